@@ -60,6 +60,7 @@ struct WaveCtl {
     int fetch_shadow;
     int error;     // media walks that exhausted their step budget in this render
     int overflow;  // traversal node groups that found the stack full (the BVH depth check keeps this 0)
+    int fetch_query;  // next ray of a ray query (follows overflow: a query clears the two together)
     unsigned long long stats[8];  // extend rays, shadow rays, ext nodes, ext tris, sh nodes, sh tris,
                                   // NaN samples, paths ended by a NaN throughput
     int bucket[kShadeBuckets];    // extend results per shade bucket
@@ -148,6 +149,7 @@ struct LaunchShape {
     int blocks_extend, blocks_shade, blocks_shadow;
     int blocks_shade_plain;  // the shade kernel without media, guiding and textures
     int blocks_sample;
+    int blocks_query;        // k_trace_queue (the closest- and any-hit builds have the same bounds)
 };
 void query_shape(LaunchShape& s);
 // The a-trous denoiser: colour, albedo and normal AOVs (W x H float4) in;
@@ -202,9 +204,10 @@ void launch_next_wave(const rtd::Ctx& c, cudaStream_t st);
 void launch_finalize(const rtd::JobDesc& host_job, const rtd::JobDesc* dev_job, cudaStream_t st);
 void launch_begin_n(const rtd::JobDesc* dev_job, int64_t npix, cudaStream_t st);
 void launch_finalize_n(const rtd::JobDesc* dev_job, int64_t npix, cudaStream_t st);
-// Per-thread ray queries; `overflow` (device int) counts traversal stack overflows.
-void launch_trace(const rtd::SceneView& sc, bool any_hit, const float* rays, int64_t n, float* hits, int* overflow,
-                  cudaStream_t st);
+// Ray queries; `overflow` (device int) counts traversal stack overflows and
+// `fetch` (device int, zero) hands the rays of a large batch out.
+void launch_trace(const rtd::SceneView& sc, const LaunchShape& s, bool any_hit, const float* rays, int64_t n,
+                  float* hits, int* overflow, int* fetch, cudaStream_t st);
 // Ray queries through the wavefront kernels: stage n rays (8 floats each, device)
 // as the extend queue (closest hit) or the shadow queue (any hit) of a wave,
 // run launch_extend / launch_shadow, then collect the hits (4 floats each, device).

@@ -942,10 +942,12 @@ rt_status rt_renderer_trace(rt_renderer* r, int32_t any_hit, const float* rays, 
     RT_ON_DEVICE(r, "rt_renderer_trace");
     if (n == 0) return RT_OK;
     int* ovf = overflow_counter(r);
+    int* fetch = ovf + 1;
+    static_assert(offsetof(WaveCtl, fetch_query) == offsetof(WaveCtl, overflow) + sizeof(int), "counter layout");
     int h_ovf = 0;
-    RT_CUDA(cudaMemsetAsync(ovf, 0, sizeof(int), r->stream), "rt_renderer_trace");
+    RT_CUDA(cudaMemsetAsync(ovf, 0, 2 * sizeof(int), r->stream), "rt_renderer_trace");
     if (device_ptrs) {
-        rth::launch_trace(r->ds.view, any_hit != 0, rays, n, hits, ovf, r->stream);
+        rth::launch_trace(r->ds.view, r->shape, any_hit != 0, rays, n, hits, ovf, fetch, r->stream);
         RT_CUDA(cudaGetLastError(), "rt_renderer_trace");
         RT_CUDA(cudaMemcpyAsync(&h_ovf, ovf, sizeof(int), cudaMemcpyDeviceToHost, r->stream), "rt_renderer_trace");
         RT_CUDA(cudaStreamSynchronize(r->stream), "rt_renderer_trace");
@@ -955,7 +957,7 @@ rt_status rt_renderer_trace(rt_renderer* r, int32_t any_hit, const float* rays, 
     RT_CUDA(dr.alloc(size_t(n) * 32), "rt_renderer_trace: allocate");
     RT_CUDA(dh.alloc(size_t(n) * 16), "rt_renderer_trace: allocate");
     RT_CUDA(cudaMemcpyAsync(dr.ptr, rays, size_t(n) * 32, cudaMemcpyHostToDevice, r->stream), "rt_renderer_trace");
-    rth::launch_trace(r->ds.view, any_hit != 0, dr.as<float>(), n, dh.as<float>(), ovf, r->stream);
+    rth::launch_trace(r->ds.view, r->shape, any_hit != 0, dr.as<float>(), n, dh.as<float>(), ovf, fetch, r->stream);
     RT_CUDA(cudaGetLastError(), "rt_renderer_trace");
     RT_CUDA(cudaMemcpyAsync(hits, dh.ptr, size_t(n) * 16, cudaMemcpyDeviceToHost, r->stream), "rt_renderer_trace");
     RT_CUDA(cudaMemcpyAsync(&h_ovf, ovf, sizeof(int), cudaMemcpyDeviceToHost, r->stream), "rt_renderer_trace");

@@ -273,7 +273,8 @@ struct TravState {
 
 // One wide node (or one postponed triangle group) and its triangles; returns
 // true when the ray is finished.  `overflows` as in traverse().
-template <bool AnyHit, bool Stats>
+// kPostpone: the triangle-postponing percentage of the warp's lanes (0: never).
+template <bool AnyHit, bool Stats, int kPostpone>
 RT_D bool trav_step(TravState& s, TravStack& st, uint32_t& nodes_visited, uint32_t& tris_tested, uint32_t& overflows) {
     uint32_t tb, tbits;
     if (s.g.x & kTriGroup) {
@@ -300,10 +301,9 @@ RT_D bool trav_step(TravState& s, TravStack& st, uint32_t& nodes_visited, uint32
     // postponing percentage of the lanes in this step still test triangles,
     // the rest of the group goes on the stack and the lane returns to node
     // traversal with the others (+7% paths/s on the 2.59M-triangle scene).
-    constexpr int kPostpone = AnyHit ? kPostponePercentAny : kPostponePercentClosest;
-    const int n_step = __popc(__activemask());
+    const int n_step = kPostpone > 0 ? __popc(__activemask()) : 0;
     while (tbits) {
-        if (__popc(__activemask()) * 100 < kPostpone * n_step && st.sp < s.tri_room) {
+        if (kPostpone > 0 && __popc(__activemask()) * 100 < kPostpone * n_step && st.sp < s.tri_room) {
             st.push(make_uint2(tb | kTriGroup, tbits));
             break;
         }
@@ -330,7 +330,7 @@ RT_D bool trav_step(TravState& s, TravStack& st, uint32_t& nodes_visited, uint32
     return false;
 }
 
-template <bool AnyHit, bool Stats, class Src>
+template <bool AnyHit, bool Stats, int kPostpone = AnyHit ? kPostponePercentAny : kPostponePercentClosest, class Src>
 RT_D void traverse_queue(Src& src, int* fetch_counter, int total, uint32_t& nodes_visited, uint32_t& tris_tested,
                          uint32_t& rays, uint32_t& overflows) {
     constexpr int kRefillLanes = AnyHit ? kRefillLanesAny : kRefillLanesClosest;
@@ -371,7 +371,7 @@ RT_D void traverse_queue(Src& src, int* fetch_counter, int total, uint32_t& node
                 }
             }
         }
-        if (active && trav_step<AnyHit, Stats>(s, st, nodes_visited, tris_tested, overflows)) {
+        if (active && trav_step<AnyHit, Stats, kPostpone>(s, st, nodes_visited, tris_tested, overflows)) {
             fin = true;
             active = false;
         }
