@@ -306,8 +306,6 @@ struct Collapser {
         int tri_off = 0;
         int next_child = 0;
         const float p[3] = {node.px, node.py, node.pz};
-        uint8_t* qlo[3] = {node.qlox, node.qloy, node.qloz};
-        uint8_t* qhi[3] = {node.qhix, node.qhiy, node.qhiz};
         for (int s = 0; s < 8; s++) {
             int c = child_at[s];
             if (c < 0) {
@@ -323,8 +321,8 @@ struct Collapser {
                 hi = std::min(255.0, std::max(0.0, hi));
                 while (lo > 0 && double(p[a]) + lo * sc > double(cn.box.lo[a])) lo -= 1;
                 while (hi < 255 && double(p[a]) + hi * sc < double(cn.box.hi[a])) hi += 1;
-                qlo[a][s] = uint8_t(lo);
-                qhi[a][s] = uint8_t(hi);
+                node.q[a][2 * s] = uint8_t(lo);
+                node.q[a][2 * s + 1] = uint8_t(hi);
             }
             if (cn.left < 0 || cn.count <= kMaxLeaf) {
                 std::vector<int> tris;
@@ -364,8 +362,6 @@ bool validate(const std::vector<rtd::CwNode>& nodes, const std::vector<int>& ord
         const rtd::CwNode& n = nodes[i];
         const float p[3] = {n.px, n.py, n.pz};
         const int e[3] = {int(n.ex) - 127, int(n.ey) - 127, int(n.ez) - 127};
-        const uint8_t* qlo[3] = {n.qlox, n.qloy, n.qloz};
-        const uint8_t* qhi[3] = {n.qhix, n.qhiy, n.qhiz};
         int rank = 0;
         for (int s = 0; s < 8; s++) {
             if (n.meta[s] == 0) {
@@ -377,8 +373,8 @@ bool validate(const std::vector<rtd::CwNode>& nodes, const std::vector<int>& ord
             }
             double lo[3], hi[3];
             for (int a = 0; a < 3; a++) {
-                lo[a] = double(p[a]) + std::ldexp(double(qlo[a][s]), e[a]);
-                hi[a] = double(p[a]) + std::ldexp(double(qhi[a][s]), e[a]);
+                lo[a] = double(p[a]) + std::ldexp(double(n.q[a][2 * s]), e[a]);
+                hi[a] = double(p[a]) + std::ldexp(double(n.q[a][2 * s + 1]), e[a]);
             }
             auto inside = [&](const float* v) {
                 for (int a = 0; a < 3; a++)

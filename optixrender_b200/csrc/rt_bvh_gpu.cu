@@ -683,8 +683,6 @@ __global__ void k_collapse(const WideItem* __restrict__ items, const int* __rest
     node.child_base = uint32_t(cb);
     node.tri_base = uint32_t(tb);
     const float p[3] = {node.px, node.py, node.pz};
-    uint8_t* qlo[3] = {node.qlox, node.qloy, node.qloz};
-    uint8_t* qhi[3] = {node.qhix, node.qhiy, node.qhiz};
     int tri_off = 0, next_child = 0;
     for (int s = 0; s < 8; s++) {
         const int c = child_at[s];
@@ -701,8 +699,8 @@ __global__ void k_collapse(const WideItem* __restrict__ items, const int* __rest
             hi = fmin(255.0, fmax(0.0, hi));
             while (lo > 0 && double(p[a]) + lo * sc > double(cn.lo[a])) lo -= 1;
             while (hi < 255 && double(p[a]) + hi * sc < double(cn.hi[a])) hi += 1;
-            qlo[a][s] = uint8_t(lo);
-            qhi[a][s] = uint8_t(hi);
+            node.q[a][2 * s] = uint8_t(lo);
+            node.q[a][2 * s + 1] = uint8_t(hi);
         }
         if (cn.left < 0 || cn.count <= kMaxLeaf) {
             const int k = cn.count;

@@ -249,8 +249,7 @@ struct __align__(16) CwNode {
     uint32_t child_base;
     uint32_t tri_base;
     uint8_t meta[8];
-    uint8_t qlox[8], qloy[8], qloz[8];
-    uint8_t qhix[8], qhiy[8], qhiz[8];
+    uint8_t q[3][16];  // per axis: the children's low and high planes in turn (slot s: q[a][2s], q[a][2s + 1])
 };
 static_assert(sizeof(CwNode) == 80, "CwNode layout");
 

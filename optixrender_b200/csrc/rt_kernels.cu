@@ -181,7 +181,7 @@ struct ExtendSrc {
     }
 };
 
-template <bool Stats>
+template <bool Stats, bool Few>
 __global__ void __launch_bounds__(kBlock, kTravMinBlocks) k_extend(Ctx c) {
     WaveCtl* ctl = c.wb.ctl;
     const int cur = c.bounce & 1, nxt = cur ^ 1;
@@ -194,7 +194,10 @@ __global__ void __launch_bounds__(kBlock, kTravMinBlocks) k_extend(Ctx c) {
     const int total = ctl->count[cur];
     uint32_t nodes = 0, tris = 0, rays = 0, overflows = 0;
     ExtendSrc src{&c, c.wb.queue[cur]};
-    traverse_queue<false, Stats>(src, &ctl->fetch_ext, total, nodes, tris, rays, overflows);
+    if (Few)
+        traverse_queue_few<false, Stats, kPostponePercentClosest>(src, &ctl->fetch_ext, total, nodes, tris, rays, overflows);
+    else
+        traverse_queue<false, Stats>(src, &ctl->fetch_ext, total, nodes, tris, rays, overflows);
     if (overflows) atomicAdd(&ctl->overflow, int(overflows));
     if (Stats) {
         warp_stat(&ctl->stats[0], rays);
@@ -764,13 +767,16 @@ struct ShadowSrc {
     }
 };
 
-template <bool Stats>
+template <bool Stats, bool Few>
 __global__ void __launch_bounds__(kBlock, kTravMinBlocks) k_shadow(Ctx c) {
     WaveCtl* ctl = c.wb.ctl;
     const int total = ctl->shadow_count[c.bounce & 1];
     uint32_t nodes = 0, tris = 0, rays = 0, overflows = 0;
     ShadowSrc src{&c};
-    traverse_queue<true, Stats>(src, &ctl->fetch_shadow, total, nodes, tris, rays, overflows);
+    if (Few)
+        traverse_queue_few<true, Stats, kPostponePercentAny>(src, &ctl->fetch_shadow, total, nodes, tris, rays, overflows);
+    else
+        traverse_queue<true, Stats>(src, &ctl->fetch_shadow, total, nodes, tris, rays, overflows);
     if (overflows) atomicAdd(&ctl->overflow, int(overflows));
     if (Stats) {
         warp_stat(&ctl->stats[1], rays);
@@ -1067,15 +1073,13 @@ __global__ void __launch_bounds__(kBlock) k_trace(SceneView sc, const float* __r
 
 // The same queries through the persistent loop with lane refill, for batches
 // of more rays than the chip holds threads (launch_trace).  Triangles are not
-// postponed, so every ray meets nodes and triangles in k_trace's order: of
+// postponed, so every ray tests triangles in k_trace's order: of
 // triangles at exactly equal distances (coplanar faces) the same one is
 // reported, and an any-hit ray reports the same triangle's distance.
-// Bound by issue slots (77% busy) at 15 of 32 threads an instruction; with a
-// thread per ray a warp ran as long as its longest ray.  2^22 rays leaving the
-// surfaces of the 2.59M-triangle scene: closest hit 4.72 -> 2.71 ms (0.89 ->
-// 1.55 Grays/s; postponing, which may change which of two coplanar triangles
-// is reported, would give 2.34 ms), 10^6 any-hit rays of finite reach 0.63 ->
-// 0.62 ms.
+// A thread per ray made a warp run as long as its longest ray: 2^22 rays
+// leaving the surfaces of the 2.59M-triangle scene 4.72 ms (0.89 Grays/s),
+// with refilled lanes 2.71 ms, with listed triangles 1.76 ms (2.4 Grays/s);
+// 10^6 any-hit rays of finite reach 0.63, 0.62 and 0.40 ms.
 struct TraceSrc {
     const SceneView* sc;
     const float4* rays;
@@ -1097,14 +1101,17 @@ struct TraceSrc {
     }
 };
 
-template <bool AnyHit>
+template <bool AnyHit, bool Few>
 __global__ void __launch_bounds__(kBlock, kTravMinBlocks) k_trace_queue(const __grid_constant__ SceneView sc,
                                                                         const float4* __restrict__ rays, int n,
                                                                         float4* __restrict__ hits, int* fetch,
                                                                         int* overflow) {
     uint32_t nodes = 0, tris = 0, count = 0, overflows = 0;
     TraceSrc src{&sc, rays, hits, AnyHit};
-    traverse_queue<AnyHit, false, 0>(src, fetch, n, nodes, tris, count, overflows);
+    if (Few)
+        traverse_queue_few<AnyHit, false, 0>(src, fetch, n, nodes, tris, count, overflows);
+    else
+        traverse_queue<AnyHit, false>(src, fetch, n, nodes, tris, count, overflows);
     if (overflows) atomicAdd(overflow, int(overflows));
 }
 
@@ -1276,17 +1283,17 @@ void query_shape(LaunchShape& s) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&s.sms, cudaDevAttrMultiProcessorCount, dev);
     int b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_extend<false>, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_extend<false, false>, kBlock, 0);
     s.blocks_extend = s.sms * (b > 0 ? b : 1);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_shade<false, true>, kBlock, 0);
     s.blocks_shade = s.sms * (b > 0 ? b : 1);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_shade<false, false>, kBlock, 0);
     s.blocks_shade_plain = s.sms * (b > 0 ? b : 1);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_shadow<false>, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_shadow<false, false>, kBlock, 0);
     s.blocks_shadow = s.sms * (b > 0 ? b : 1);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_sample<false>, kBlock, 0);
     s.blocks_sample = s.sms * (b > 0 ? b : 1);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_trace_queue<false>, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_trace_queue<false, false>, kBlock, 0);
     s.blocks_query = s.sms * (b > 0 ? b : 1);
 }
 
@@ -1331,10 +1338,9 @@ void destroy_fork(WaveFork& f) {
 
 void launch_raygen(const Ctx& c, cudaStream_t st) { k_raygen<<<grid_for(c.wb.capacity, kRaygenBlock), kRaygenBlock, 0, st>>>(c); }
 void launch_extend(const Ctx& c, const LaunchShape& s, bool stats, cudaStream_t st) {
-    if (stats)
-        k_extend<true><<<s.blocks_extend, kBlock, 0, st>>>(c);
-    else
-        k_extend<false><<<s.blocks_extend, kBlock, 0, st>>>(c);
+    auto* k = c.few_nodes ? (stats ? k_extend<true, true> : k_extend<false, true>)
+                          : (stats ? k_extend<true, false> : k_extend<false, false>);
+    k<<<s.blocks_extend, kBlock, 0, st>>>(c);
 }
 void launch_shade(const Ctx& c, const LaunchShape& s, bool stats, cudaStream_t st) {
     const bool full = c.features != 0;
@@ -1358,10 +1364,9 @@ void launch_sample(const Ctx& c, const LaunchShape& s, bool stats, cudaStream_t 
         k_sample<false><<<s.blocks_sample, kBlock, 0, st>>>(c);
 }
 void launch_shadow(const Ctx& c, const LaunchShape& s, bool stats, cudaStream_t st) {
-    if (stats)
-        k_shadow<true><<<s.blocks_shadow, kBlock, 0, st>>>(c);
-    else
-        k_shadow<false><<<s.blocks_shadow, kBlock, 0, st>>>(c);
+    auto* k = c.few_nodes ? (stats ? k_shadow<true, true> : k_shadow<false, true>)
+                          : (stats ? k_shadow<true, false> : k_shadow<false, false>);
+    k<<<s.blocks_shadow, kBlock, 0, st>>>(c);
 }
 void launch_resolve(const Ctx& c, cudaStream_t st) {
     // enough threads for a few items each on the benchmark frame (2M pixels)
@@ -1404,10 +1409,9 @@ void launch_trace(const SceneView& sc, const LaunchShape& s, bool any_hit, const
     if (n > int64_t(s.blocks_query) * kBlock && n <= (int64_t(1) << 30)) {
         const float4* r4 = reinterpret_cast<const float4*>(rays);
         float4* h4 = reinterpret_cast<float4*>(hits);
-        if (any_hit)
-            k_trace_queue<true><<<s.blocks_query, kBlock, 0, st>>>(sc, r4, int(n), h4, fetch, overflow);
-        else
-            k_trace_queue<false><<<s.blocks_query, kBlock, 0, st>>>(sc, r4, int(n), h4, fetch, overflow);
+        auto* k = few_nodes(sc) ? (any_hit ? k_trace_queue<true, true> : k_trace_queue<false, true>)
+                                : (any_hit ? k_trace_queue<true, false> : k_trace_queue<false, false>);
+        k<<<s.blocks_query, kBlock, 0, st>>>(sc, r4, int(n), h4, fetch, overflow);
         return;
     }
     if (any_hit)

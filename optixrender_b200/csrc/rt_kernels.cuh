@@ -124,7 +124,16 @@ struct Ctx {
     int max_depth;  // largest max_depth of the jobs in the wave
     rtg::GuideCtx G;  // path guiding (G.mix null: not guided)
     int features;     // kFeature* bits of the wave's scenes and jobs (host side: picks the shade kernel)
+    int few_nodes;    // few_nodes() of all the wave's scenes (host side: picks the traversal loop)
 };
+
+// Scenes whose rays visit a node or two and test triangles at each of them are
+// traversed by traverse_queue_few, larger ones by traverse_queue.  k_extend +
+// k_shadow, 640 x 640 at 8 spp, few / large: 3 nodes 1.36 / 1.87 ms, 149 nodes
+// 2.09 / 2.31 ms, 729 nodes 2.69 / 2.66 ms, 1001 nodes 3.47 / 3.29 ms, 3254
+// nodes 3.01 / 2.86 ms.
+constexpr int kFewNodes = 512;
+inline bool few_nodes(const SceneView& sc) { return sc.num_nodes <= kFewNodes; }
 
 // Scene and job features that need the full shade kernel.
 constexpr int kFeatureMedia = 1, kFeatureGuide = 2, kFeatureTextures = 4;

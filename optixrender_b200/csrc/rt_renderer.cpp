@@ -663,6 +663,7 @@ rt_status rt_renderer_render(rt_renderer* r) {
     c.max_depth = o.max_depth;
     c.features = (r->ds.view.num_media > 0 ? kFeatureMedia : 0) | (guided ? kFeatureGuide : 0) |
                  (r->ds.view.num_tex > 0 ? kFeatureTextures : 0);
+    c.few_nodes = few_nodes(r->ds.view);
     rtg::NetView net{};
     if (guided) {
         float3 lo, inv;
@@ -1013,6 +1014,7 @@ rt_status rt_renderer_trace_wavefront(rt_renderer* r, int32_t any_hit, const flo
     c.wave_ring = 1;
     c.bounce = 0;
     c.max_depth = 1;
+    c.few_nodes = few_nodes(r->ds.view);
     const bool stats = counters != nullptr;
     int overflows = 0;
     for (int64_t b0 = 0; b0 < n; b0 += chunk) {

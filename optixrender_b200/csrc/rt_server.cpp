@@ -106,6 +106,7 @@ struct rt_server {
     std::vector<std::unique_ptr<DeviceScene>> scenes;
     std::vector<SceneGuide> guides;  // one per scene; networks created at the first guided wave
     int64_t scene_bytes = 0;
+    bool few = true;                  // few_nodes() of every resident scene
     std::vector<int> scene_features;  // per scene: kFeatureMedia / kFeatureTextures
     std::map<int64_t, std::unique_ptr<Job>> jobs;
     std::deque<int64_t> queued;
@@ -276,6 +277,7 @@ Ctx make_ctx(rt_server* s, int group) {
     c.wave_ring = s->ring_size;
     c.max_depth = s->opt.max_depth;
     c.features = group == kGroupPlain ? 0 : group == kGroupFull ? kFeatureMedia | kFeatureTextures : kFeatureGuide;
+    c.few_nodes = s->few;
     if (gscene >= 0) {
         const SceneGuide& g = s->guides[size_t(gscene)];
         c.G.mix = s->g_mix.as<rtg::Mixture>();
@@ -704,6 +706,12 @@ rt_status rt_server_add_scene(rt_server* s, const rt_scene* scene, int32_t* id) 
         SV_CUDA(s->mat_tex.alloc(size_t(s->capacity) * sizeof(DevMaterial)), "allocate textured materials");
         for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);  // captured without the buffer
         s->graphs.clear();
+    }
+    if (s->few && !few_nodes(ds->view)) {
+        SV_CUDA(cudaStreamSynchronize(s->stream), "rt_server_add_scene");
+        for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);  // captured with the other traversal loop
+        s->graphs.clear();
+        s->few = false;
     }
     s->scene_features.push_back((ds->view.num_media > 0 ? kFeatureMedia : 0) |
                                 (ds->view.num_tex > 0 ? kFeatureTextures : 0));

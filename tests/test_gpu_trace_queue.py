@@ -66,3 +66,23 @@ def test_batches_around_the_line_between_the_two_loops():
     for blocks in range(1, 17):  # the line is at a whole number of blocks per multiprocessor
         for n in (sms * blocks * 128 - 1, sms * blocks * 128, sms * blocks * 128 + 1):
             assert np.array_equal(r.trace(rays[:n], any_hit=True).view(np.int32), full[:n].view(np.int32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("any_hit", [False, True])
+def test_more_triangles_at_a_step_than_the_warps_list_holds(any_hit):
+    """Thousands of large triangles through each other: every node a ray visits has most of its leaves hit, so a
+    step brings several hundred triangles where the list holds 128, and rays keep the rest for later steps."""
+    torch = pytest.importorskip("torch")
+    g = np.random.default_rng(5)
+    tri = (g.uniform(-1, 1, (6000, 1, 3)) + g.uniform(-1.5, 1.5, (6000, 3, 3))).astype(np.float32)
+    s = rt.Scene()
+    s.add_mesh(tri.reshape(-1, 3), rt.material(rt.MAT_DIFFUSE))
+    r = rt.Renderer(s, rt.options(width=4, height=4))
+    n = (1 << 19) + 5
+    part = 128 * torch.cuda.get_device_properties(0).multi_processor_count
+    rays = _rays(n, 21)
+    whole = r.trace(rays, any_hit=any_hit)
+    parts = np.concatenate([r.trace(rays[i:i + part], any_hit=any_hit) for i in range(0, n, part)])
+    assert (whole[:, 3].view(np.int32) >= 0).mean() > 0.1
+    assert np.array_equal(whole.view(np.int32), parts.view(np.int32))
