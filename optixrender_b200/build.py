@@ -29,7 +29,10 @@ NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-ftz=true", "-prec-div=false", 
 CXX_FLAGS = ["-std=c++17", "-O2", "-fPIC", "-ffp-contract=off", "-fopenmp", "-Wall", "-Wno-unused-function", "-Wno-unknown-pragmas",
              "-I/usr/local/cuda/include"]
 
-CU_SOURCES = ["rt_kernels.cu", "rt_trace_scratch.cu", "rt_guide.cu", "rt_guide_api.cu", "rt_bvh_gpu.cu"]
+# sources whose results must equal the host's: denormals kept, divisions rounded, no contraction
+HOST_MATH = {"rt_scene_gpu.cu": ["-ftz=false", "-prec-div=true", "-prec-sqrt=true", "-fmad=false"]}
+
+CU_SOURCES = ["rt_kernels.cu", "rt_trace_scratch.cu", "rt_guide.cu", "rt_guide_api.cu", "rt_bvh_gpu.cu", "rt_scene_gpu.cu"]
 CPP_SOURCES = ["rt_capi.cpp", "rt_renderer.cpp", "rt_bvh.cpp", "rt_tables.cpp", "rt_scene_io.cpp", "rt_server.cpp",
                "rt_png.cpp", "rt_jpeg.cpp"]
 HEADERS = ["rt_device.cuh", "rt_shading.cuh", "rt_traverse.cuh", "rt_kernels.cuh", "rt_internal.h", "rt_bvh.h",
@@ -65,7 +68,10 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
         o = BUILD / (src + ".o")
         objs.append(o)
         if force or not _newer(o, [s] + headers):
-            jobs.append([NVCC] + ARCH + NVCC_FLAGS + ["-c", str(s), "-o", str(o)])
+            flags = NVCC_FLAGS
+            if src in HOST_MATH:
+                flags = [f for f in NVCC_FLAGS if not f.startswith(("-ftz", "-prec-"))] + HOST_MATH[src]
+            jobs.append([NVCC] + ARCH + flags + ["-c", str(s), "-o", str(o)])
     for src in CPP_SOURCES:
         s = CSRC / src
         if not s.exists():

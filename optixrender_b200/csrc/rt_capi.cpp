@@ -332,6 +332,8 @@ rt_status rt_scene_add_mesh(rt_scene* s, const rt_mesh_desc* m, const rt_materia
                 }
             }
         }
+        s->own_normals = s->own_normals || m->normals;
+        s->own_texcoords = s->own_texcoords || m->texcoords;
         s->mesh_mat.push_back(*mat);
         s->mesh_out.push_back(out_medium);
         s->mesh_in.push_back(in_medium);

@@ -16,6 +16,9 @@ struct rt_scene {
     std::vector<float> tv;   // 9 floats per triangle
     std::vector<float> tn;   // 9 floats per triangle
     std::vector<float> tuv;  // 6 floats per triangle
+    // any mesh brought its own; without, tn holds face normals and tuv the
+    // default coordinates, and an upload derives them from the positions
+    bool own_normals = false, own_texcoords = false;
     std::vector<int> tri_mesh;
     std::vector<rt_material> mesh_mat;
     std::vector<int> mesh_out, mesh_in;

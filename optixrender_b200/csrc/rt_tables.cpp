@@ -86,6 +86,17 @@ void kulla_conty_tables(float* bsdf, float* avg) {
     }
 }
 
+// The sum of the image's luminances, in pixel order.
+float env_luminance_sum(const float* img, int w, int h) {
+    const size_t n = size_t(w) * h;
+    float sum = 0.0f;
+    for (size_t q = 0; q < n; q++) {
+        const float* p = img + q * 4;
+        sum += 0.299f * p[0] + 0.587f * p[1] + 0.114f * p[2];
+    }
+    return sum;
+}
+
 // HdrTexture::CalculateHdrCache, core/src/Scene.cpp:217-313: luminance pdf,
 // column marginal and per-column conditional CDFs, and a w x h table mapping a
 // uniform (u, v) to a texel by inverse-CDF lookups; texel (i, j) stores
