@@ -38,17 +38,6 @@ RT_D int warp_fetch(int* counter, int lane) {
     return __shfl_sync(0xffffffffu, base, 0);
 }
 
-// Appends `flag` lanes of a converged warp to a queue; returns the position.
-RT_D int warp_append(int* counter, bool flag, int lane) {
-    unsigned m = __ballot_sync(0xffffffffu, flag);
-    if (m == 0) return -1;
-    int leader = __ffs(m) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(counter, __popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    return flag ? base + __popc(m & ((1u << lane) - 1u)) : -1;
-}
-
 RT_D void warp_stat(unsigned long long* dst, unsigned v) {
     unsigned long long x = v;
 #pragma unroll
@@ -281,9 +270,7 @@ __global__ void __launch_bounds__(kBlock) k_shade(Ctx c) {
         prefix[kShadeBuckets] = acc;
     }
     __syncthreads();
-    while (true) {
-        int base = warp_fetch(&ctl->fetch_shade, lane);
-        if (base >= total) break;
+    for (int base = warp_fetch(&ctl->fetch_shade, lane); base < total;) {
         int i = base + lane;
         bool cont = false, defer = false;
         bool sh0 = false, sh1 = false;
@@ -637,16 +624,28 @@ __global__ void __launch_bounds__(kBlock) k_shade(Ctx c) {
                 B.thr[slot] = f4(history, pre_pdf);
             }
         }
-        int qp = warp_append(&ctl->count[nxt], cont, lane);
+        // The next items and the places in the three queues come from one atomic
+        // instruction of four lanes: one after the other, each was a round trip
+        // to L2 of its own in a kernel that mostly waits for memory.
+        const unsigned mc = __ballot_sync(0xffffffffu, cont), md = __ballot_sync(0xffffffffu, defer);
+        const unsigned m0 = __ballot_sync(0xffffffffu, sh0), m1 = __ballot_sync(0xffffffffu, sh1);
+        int* counter = lane == 0 ? &ctl->fetch_shade
+                       : lane == 1 ? &ctl->count[nxt] : lane == 2 ? &ctl->sample_count : &ctl->shadow_count[cur];
+        const int add = lane == 0 ? 32 : lane == 1 ? __popc(mc) : lane == 2 ? __popc(md) : __popc(m0) + __popc(m1);
+        int got = 0;
+        if (lane < 4 && add != 0) got = atomicAdd(counter, add);
+        base = __shfl_sync(0xffffffffu, got, 0);
+        const unsigned below = (1u << lane) - 1u;
+        const int qp = __shfl_sync(0xffffffffu, got, 1) + __popc(mc & below);
         if (cont) B.queue[nxt][qp] = slot;
-        int sp = warp_append(&ctl->sample_count, defer, lane);
+        const int sp = __shfl_sync(0xffffffffu, got, 2) + __popc(md & below);
         if (defer) B.squeue[sp] = slot;
-        int p0 = warp_append(&ctl->shadow_count[cur], sh0, lane);
+        const int sh = __shfl_sync(0xffffffffu, got, 3), p0 = sh + __popc(m0 & below);
         if (sh0) {
             B.sh_o[p0] = f4(s0o, s0t);
             B.sh_d[p0] = f4(s0d, __int_as_float(slot * 2 + 0));
         }
-        int p1 = warp_append(&ctl->shadow_count[cur], sh1, lane);
+        const int p1 = sh + __popc(m0) + __popc(m1 & below);
         if (sh1) {
             B.sh_o[p1] = f4(s1o, s1t);
             B.sh_d[p1] = f4(s1d, __int_as_float(slot * 2 + 1));
@@ -683,9 +682,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_sample(Ctx c) {
     const WaveParams& W = wave_of(c);
     const int lane = threadIdx.x & 31;
     uint32_t nan_paths = 0;
-    while (true) {
-        const int base = warp_fetch(&ctl->fetch_sample, lane);
-        if (base >= total) break;
+    for (int base = warp_fetch(&ctl->fetch_sample, lane); base < total;) {
         const int i = base + lane;
         bool cont = false;
         int slot = 0;
@@ -738,7 +735,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_sample(Ctx c) {
                 B.thr[slot] = f4(history, bpdf);
             }
         }
-        const int qp = warp_append(&ctl->count[nxt], cont, lane);
+        // the next items and the places in the queue from one atomic instruction (as in k_shade)
+        const unsigned mc = __ballot_sync(0xffffffffu, cont);
+        const int add = lane == 0 ? 32 : __popc(mc);
+        int got = 0;
+        if (lane < 2 && add != 0) got = atomicAdd(lane == 0 ? &ctl->fetch_sample : &ctl->count[nxt], add);
+        base = __shfl_sync(0xffffffffu, got, 0);
+        const int qp = __shfl_sync(0xffffffffu, got, 1) + __popc(mc & ((1u << lane) - 1u));
         if (cont) B.queue[nxt][qp] = slot;
     }
     if (Stats) warp_stat(&ctl->stats[7], nan_paths);
