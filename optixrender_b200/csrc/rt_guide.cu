@@ -187,7 +187,7 @@ RT_D void level_corners(int res, float3 x, Corners& c) {
     // directly, a finer one hashes them.  Branching (rather than selecting
     // per corner) spares the dense levels the hash arithmetic; the condition
     // is the same for every lane on the same level.
-    if (uint64_t(r1) * r1 * r1 <= uint64_t(kT)) {
+    if (dense_level(res)) {
         const uint32_t r2 = r1 * r1, base = ix + iy * r1 + iz * r2;
 #pragma unroll
         for (int k = 0; k < 8; k++) c.idx[k] = base + (k & 1) + ((k >> 1) & 1) * r1 + ((k >> 2) & 1) * r2;
@@ -213,6 +213,28 @@ RT_D uint32_t encode_level(const __half2* __restrict__ table, int res, int l, fl
         float2 v = __half22float2(__ldg(t + c.idx[k]));
         f0 += c.w[k] * v.x;
         f1 += c.w[k] * v.y;
+    }
+    return pack_h2(f0, f1);
+}
+
+// The same from the quads of a dense level: the same corners, weights and order
+// of the sums, in two 16-byte loads instead of eight 4-byte ones.
+RT_D uint32_t encode_level_quads(const uint4* __restrict__ quads, int res, float3 x) {
+    const float fr = float(res);
+    float px = x.x * fr, py = x.y * fr, pz = x.z * fr;
+    float cx = fminf(floorf(px), fr - 1.0f), cy = fminf(floorf(py), fr - 1.0f), cz = fminf(floorf(pz), fr - 1.0f);
+    const float fx = px - cx, fy = py - cy, fz = pz - cz;
+    const uint32_t r = uint32_t(res), r2 = r * r, at = uint32_t(cx) + uint32_t(cy) * r + uint32_t(cz) * r2;
+    const uint4 a = __ldg(quads + at), b = __ldg(quads + at + r2);
+    const uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    float f0 = 0.f, f1 = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const float w =
+            ((k & 1) ? fx : 1.0f - fx) * (((k >> 1) & 1) ? fy : 1.0f - fy) * (((k >> 2) & 1) ? fz : 1.0f - fz);
+        const float2 t = unpack_h2(v[k]);
+        f0 += w * t.x;
+        f1 += w * t.y;
     }
     return pack_h2(f0, f1);
 }
@@ -494,39 +516,47 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 2) k_guide_backward(NetView ne
 // Items of the sorted shade queue whose material type is guided, in bucket order.
 struct GuidedItems {
     int bucket[kShadeBucketsG], count[kShadeBucketsG], n;
+    int first[kShadeBucketsG];  // place of the bucket's first item in the whole queue
 };
 
 RT_D GuidedItems guided_items(const rtd::WaveCtl* ctl) {
     GuidedItems gi;
     int m = 0;  // a constant at every step once both loops are unrolled, so gi stays in registers
     gi.n = 0;
+    int before = 0;
 #pragma unroll
     for (int b = 0; b < rtd::kShadeBuckets; b++) {
+        const int count = ctl->bucket[b];
+        before += count;
         if (b == rtd::kMissBucket || !guided_type(b)) continue;
         gi.bucket[m] = b;
-        gi.count[m] = ctl->bucket[b];
+        gi.count[m] = count;
+        gi.first[m] = before - count;
         gi.n += gi.count[m];
         m++;
     }
 #pragma unroll
-    for (; m < kShadeBucketsG; m++) gi.bucket[m] = gi.count[m] = 0;
+    for (; m < kShadeBucketsG; m++) gi.bucket[m] = gi.count[m] = gi.first[m] = 0;
     return gi;
 }
 
-// The slot of guided item i: bucket m holds items [base_m, base_m + count_m).
-// Unrolled with constant indices (a runtime index would put gi in local memory).
-RT_D int guided_slot(const GuidedItems& gi, const rtd::WaveBufs& B, int i) {
-    int bucket = gi.bucket[0], base = 0;
+// The slot of guided item i and its place in the whole queue: bucket m holds
+// items [base_m, base_m + count_m).  Unrolled with constant indices (a runtime
+// index would put gi in local memory).
+RT_D int guided_slot(const GuidedItems& gi, const rtd::WaveBufs& B, int i, int& place) {
+    int bucket = gi.bucket[0], base = 0, first = gi.first[0];
     bool found = false;
 #pragma unroll
     for (int m = 0; m < kShadeBucketsG - 1; m++) {
         if (!found && i >= base + gi.count[m]) {
             base += gi.count[m];
             bucket = gi.bucket[m + 1];
+            first = gi.first[m + 1];
         } else {
             found = true;
         }
     }
+    place = first + (i - base);
     return B.sorted[size_t(bucket) * size_t(B.capacity) + size_t(i - base)];
 }
 
@@ -650,7 +680,13 @@ RT_D void tc_load_weights(const __half* __restrict__ mlp, unsigned char* sm) {
 RT_D void tc_encode_row(const NetView& net, float3 x, bool valid, unsigned char* sm, int row) {
     uint32_t f[kLevels];
 #pragma unroll
-    for (int l = 0; l < kLevels; l++) f[l] = valid ? encode_level(net.table, net.res[l], l, x) : 0u;
+    for (int l = 0; l < kLevels; l++) {
+        f[l] = 0u;
+        if (!valid) continue;
+        f[l] = net.quads != nullptr && net.quad_off[l] != kNoQuads
+                   ? encode_level_quads(net.quads + net.quad_off[l], net.res[l], x)
+                   : encode_level(net.table, net.res[l], l, x);
+    }
 #pragma unroll
     for (int j = 0; j < kIn / 8; j++)
         *reinterpret_cast<uint4*>(sm + kTcA + tc_off(row, 8 * j, kIn)) =
@@ -949,8 +985,31 @@ __global__ void __launch_bounds__(kTcRows) k_guide_forward_tc(NetView net, const
     tc_teardown(tmem, ok);
 }
 
+// The quads of the dense levels (NetView::quads) from the table as it is:
+// blockIdx.y is the level.
+__global__ void __launch_bounds__(256) k_guide_quads(NetView net, uint4* __restrict__ quads) {
+    const int l = blockIdx.y;
+    uint32_t off = kNoQuads;
+    int res = 0;
+#pragma unroll
+    for (int k = 0; k < kLevels; k++)
+        if (k == l) off = net.quad_off[k], res = net.res[k];
+    if (off == kNoQuads) return;
+    const uint32_t r = uint32_t(res), r1 = r + 1u, n = r * r * r1;
+    const uint32_t* t = reinterpret_cast<const uint32_t*>(net.table) + size_t(l) * kT;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t ix = i % r, iy = i / r % r, iz = i / (r * r), at = ix + iy * r1 + iz * r1 * r1;
+        quads[off + i] = make_uint4(t[at], t[at + 1u], t[at + r1], t[at + r1 + 1u]);
+    }
+}
+
 // Mixtures of this bounce's guided vertices (surface hits of guided material
-// types), written per slot for the shade kernel.
+// types), written by queue item for the shade kernel.  Bound by the L1 pipe
+// (65% of its wavefronts) and the latency of the dependent loads at 4 CTAs per
+// SM.  4.2M vertices of the 512 x 512 portal: 1.20 ms with eight 4-byte
+// gathers a level and 160-byte mixtures by slot (74%), 0.77 ms with the quads
+// of the dense levels (8 -> 2 loads) and the mixtures in planes; the shade
+// kernel that reads them 0.80 -> 0.69 ms.
 __global__ void __launch_bounds__(kTcRows) k_guide_infer_tc(rtd::Ctx c, NetView net) {
     extern __shared__ __align__(1024) unsigned char sm[];
     const uint32_t tmem = tc_setup(net, sm);
@@ -963,14 +1022,19 @@ __global__ void __launch_bounds__(kTcRows) k_guide_infer_tc(rtd::Ctx c, NetView 
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
         const int r = t * kTcRows + int(threadIdx.x);
         const bool valid = r < n;
-        const int slot = valid ? guided_slot(gi, B, r) : 0;
+        int place = 0;
+        const int slot = valid ? guided_slot(gi, B, r, place) : 0;
         tc_encode_row(net, valid ? hit_position(c, slot) : make_float3(0.f, 0.f, 0.f), valid, sm, threadIdx.x);
         float out[kOut];
         ok = tc_mlp(sm, tmem, parity, out);
         if (ok && valid) {
             Mixture m;
             head_from_outputs(out, m, net.kappa_hi);
-            c.G.mix[slot] = m;
+            float4* to = c.G.mix + place;
+#pragma unroll
+            for (int k = 0; k < kLobes; k++) to[size_t(k) * c.G.mix_stride] = m.lobe[k];
+            to[size_t(kLobes) * c.G.mix_stride] = make_float4(m.w[0], m.w[1], m.w[2], m.w[3]);
+            to[size_t(kLobes + 1) * c.G.mix_stride] = make_float4(m.w[4], m.w[5], m.w[6], m.w[7]);
         }
     }
     tc_teardown(tmem, ok);
@@ -1133,7 +1197,7 @@ __global__ void k_guide_pdf_sample(const Mixture* __restrict__ mix, const float*
                                    float* __restrict__ pdf) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const Mixture* m = mix + i;
+    const MixtureAt m = mixture_at(mix + i);
     rtd::v3 d;
     if (u) {
         d = mixture_sample(m, u[3 * i], u[3 * i + 1], u[3 * i + 2]);
@@ -1206,6 +1270,21 @@ void launch_backward(const rtg::NetView& net, const float* pos, const float* dir
         rtg::k_guide_wgrad_tc<<<(tiles + chunk - 1) / chunk, rtg::kWgWarps * 32, rtg::kWgSmem, st>>>(frags, tiles,
                                                                                                     chunk, grad_mlp);
     }
+}
+
+size_t quad_layout(rtg::NetView& net) {
+    uint64_t n = 0;
+    for (int l = 0; l < rtg::kLevels; l++) {
+        const uint64_t r = uint64_t(net.res[l]);
+        net.quad_off[l] = rtg::dense_level(net.res[l]) ? uint32_t(n) : rtg::kNoQuads;
+        if (rtg::dense_level(net.res[l])) n += r * r * (r + 1u);
+    }
+    return size_t(n) * sizeof(uint4);
+}
+
+void launch_quads(const rtg::NetView& net, int sms, cudaStream_t st) {
+    if (net.quads == nullptr) return;
+    rtg::k_guide_quads<<<dim3(unsigned(sms), rtg::kLevels), 256, 0, st>>>(net, const_cast<uint4*>(net.quads));
 }
 
 void launch_infer(const rtd::Ctx& c, const rtg::NetView& net, int sms, cudaStream_t st) {

@@ -43,12 +43,30 @@ struct NetView {
     float3 lo, inv_ext;    // position normalisation: (x - lo) * inv_ext in [0, 1]
     int res[kLevels];      // grid resolution of each level
     float kappa_hi;        // highest log-concentration of a lobe
+    // The densely indexed levels once more as quads (null: not there): entry
+    // quad_off[l] + ix + iy res + iz res^2 holds the grid points (ix, iy),
+    // (ix + 1, iy), (ix, iy + 1), (ix + 1, iy + 1) of plane iz <= res, so that
+    // a cell's eight corners are two 16-byte loads (k_guide_quads).
+    const uint4* quads;
+    uint32_t quad_off[kLevels];  // kNoQuads: a hashed level
 };
+constexpr uint32_t kNoQuads = 0xFFFFFFFFu;
+// A level whose (res + 1)^3 grid points fit the table indexes them directly.
+RT_HD bool dense_level(int res) {
+    const uint64_t r1 = uint64_t(res) + 1u;
+    return r1 * r1 * r1 <= uint64_t(kT);
+}
 
 // Guiding state of a wave, read by the wavefront kernels.
 constexpr int kGuideRec = 3;  // training records per path (the first bounces)
 struct GuideCtx {
-    Mixture* mix;        // per slot: this bounce's mixture (null: the wave is not guided)
+    // This bounce's mixtures (null: the wave is not guided) in ten planes of
+    // mix_stride float4, lobes 0..7 and the weights, by item of the sorted
+    // shade queue: the lanes of a warp of k_guide_infer_tc and of k_shade have
+    // consecutive items, so each plane is read and written in whole lines.
+    // One 160-byte record per slot cost a warp 32 L1 wavefronts per 16 bytes.
+    float4* mix;
+    size_t mix_stride;
     float4* rec;         // training records, [kGuideRec][4][capacity] float4 (null: no training)
     float prob;          // probability of sampling the mixture at a guided vertex
     float min_rough;     // conductors and clear coats rougher than this are guided
@@ -124,22 +142,27 @@ RT_D rtd::v3 vmf_sample(float4 l, float u1, float u2) {
     return normalize(t1 * (s * cp) + t2 * (s * sp) + mu * w);
 }
 
-// Density and sampling of a mixture in global memory (read-only for the kernel).
-RT_D float mixture_pdf(const Mixture* m, rtd::v3 d) {
-    const float4* w4 = reinterpret_cast<const float4*>(m->w);
-    const float4 wa = __ldg(w4), wb = __ldg(w4 + 1);
+// A mixture in global memory (read-only for the kernel): float4 k of it at
+// p[k * stride].
+struct MixtureAt {
+    const float4* p;
+    size_t stride;
+    RT_D float4 at(int k) const { return __ldg(p + size_t(k) * stride); }
+};
+RT_D MixtureAt mixture_at(const Mixture* m) { return MixtureAt{m->lobe, 1}; }
+RT_D float mixture_pdf(MixtureAt m, rtd::v3 d) {
+    const float4 wa = m.at(kLobes), wb = m.at(kLobes + 1);
     const float w[kLobes] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
     float p = 0.0f;
 #pragma unroll
-    for (int k = 0; k < kLobes; k++) p += w[k] * vmf_pdf(__ldg(m->lobe + k), d);
+    for (int k = 0; k < kLobes; k++) p += w[k] * vmf_pdf(m.at(k), d);
     return p;
 }
 // Picks a lobe with u0 and samples it with (u1, u2).
-RT_D rtd::v3 mixture_sample(const Mixture* m, float u0, float u1, float u2) {
-    const float4* w4 = reinterpret_cast<const float4*>(m->w);
-    const float4 wa = __ldg(w4), wb = __ldg(w4 + 1);
+RT_D rtd::v3 mixture_sample(MixtureAt m, float u0, float u1, float u2) {
+    const float4 wa = m.at(kLobes), wb = m.at(kLobes + 1);
     const float w[kLobes] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-    return vmf_sample(__ldg(m->lobe + pick_lobe(w, u0)), u1, u2);
+    return vmf_sample(m.at(pick_lobe(w, u0)), u1, u2);
 }
 
 // Network input of a surface point: the position moved by kSideOffset (in

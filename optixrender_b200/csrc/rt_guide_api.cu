@@ -83,6 +83,8 @@ rtg::NetView view(const rt_guide* g) {
     v.inv_ext = make_float3(1.f, 1.f, 1.f);
     for (int l = 0; l < rtg::kLevels; l++) v.res[l] = g->res[l];
     v.kappa_hi = g->opt.max_log_kappa;
+    v.quads = nullptr;
+    for (int l = 0; l < rtg::kLevels; l++) v.quad_off[l] = rtg::kNoQuads;
     return v;
 }
 

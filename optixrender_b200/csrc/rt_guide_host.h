@@ -23,6 +23,11 @@ size_t frag_bytes_per_tile();
 void launch_backward(const rtg::NetView& net, const float* pos, const float* dir, const float* weight, int n,
                      float scale, const float* weight_sum, float* grad_table, float* grad_mlp, float* loss,
                      uint32_t* frags, int frag_tiles, int sms, cudaStream_t st);
+// Lays the quads of the dense levels out (NetView::quad_off) and returns their
+// bytes; launch_quads fills net.quads from the table (nothing when null).  A
+// guided wave does it first, so the quads are never older than the table.
+size_t quad_layout(rtg::NetView& net);
+void launch_quads(const rtg::NetView& net, int sms, cudaStream_t st);
 // Renderer side: mixtures of a bounce's guided vertices, training samples of
 // a wave, training batches (strided subsets from a random start).
 void launch_infer(const rtd::Ctx& c, const rtg::NetView& net, int sms, cudaStream_t st);

@@ -391,14 +391,14 @@ __global__ void __launch_bounds__(kBlock) k_shade(Ctx c) {
                     B.aov_n[slot] = make_float2(0.f, 0.f);
                 }
             }
-            const rtg::Mixture* gmix = nullptr;
+            rtg::MixtureAt gmix{nullptr, 0};
             if (Full && G.mix != nullptr && tri >= 0 && s.mat != nullptr) {
                 const float* mw = reinterpret_cast<const float*>(s.mat);  // type, roughness (plain loads)
                 const int mtype = __float_as_int(mw[0]);
                 const bool glossy = mtype == RT_MAT_CONDUCTOR || mtype == RT_MAT_CLEARCOATED_CONDUCTOR;
                 if (rtg::guided_type(mtype) && (!glossy || mw[4] >= G.min_rough)) {
                     gp = G.prob;
-                    gmix = G.mix + slot;
+                    gmix = rtg::MixtureAt{G.mix + i, G.mix_stride};
                 }
             }
             // ---- analytic lights (devicePrograms.cu:270-271)

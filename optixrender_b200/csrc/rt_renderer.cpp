@@ -272,12 +272,13 @@ struct rt_renderer {
     // path guiding
     float lo[3] = {0.f, 0.f, 0.f}, hi[3] = {1.f, 1.f, 1.f};  // scene bounds
     rt_guide* guide = nullptr;
-    DevBuf g_mix, g_rec, g_buf, g_count, g_bpos, g_bdir, g_bw, g_wsum;
+    DevBuf g_mix, g_quads, g_rec, g_buf, g_count, g_bpos, g_bdir, g_bw, g_wsum;
     int g_cap = 0;             // slots covered by g_mix
     int64_t guide_trained = 0; // samples per pixel rendered while training
     uint32_t guide_seed = 1;
     bool graph_guided = false;
     const void* graph_mix = nullptr;
+    rtg::NetView graph_net{};  // the network view the graph's kernels were captured with
     // Pinned staging of each Render()'s launch parameters and wave table, so
     // that their copies are true asynchronous DMA; a ring, so that the host
     // can queue a few frames ahead before it waits for a buffer's last copy.
@@ -391,6 +392,13 @@ int auto_capacity(const rt_options& o, int64_t npix, int64_t total, int64_t allo
                                                            int64_t(fr / 4) / 400));
     }
     return int(clamp(cap));
+}
+
+// Whether kernels captured with one view of a guiding network serve the other.
+bool same_network(const rtg::NetView& a, const rtg::NetView& b) {
+    return a.table == b.table && a.mlp == b.mlp && a.quads == b.quads && a.kappa_hi == b.kappa_hi &&
+           std::memcmp(&a.lo, &b.lo, sizeof(a.lo)) == 0 && std::memcmp(&a.inv_ext, &b.inv_ext, sizeof(a.inv_ext)) == 0 &&
+           std::memcmp(a.res, b.res, sizeof(a.res)) == 0 && std::memcmp(a.quad_off, b.quad_off, sizeof(a.quad_off)) == 0;
 }
 
 // Guiding network and its per-slot buffers: mixtures for `cap` slots, and
@@ -694,7 +702,13 @@ rt_status rt_renderer_render(rt_renderer* r) {
             (&inv.x)[a] = 1.0f / (1.02f * ext);
         }
         net = guide_view(r->guide, lo, inv);
-        c.G.mix = r->g_mix.as<rtg::Mixture>();
+        const size_t quad_bytes = rtgh::quad_layout(net);
+        if (r->g_quads.alloc(quad_bytes) == cudaSuccess)
+            net.quads = r->g_quads.as<uint4>();
+        else
+            cudaGetLastError();  // no room: the inference reads the table itself
+        c.G.mix = r->g_mix.as<float4>();
+        c.G.mix_stride = size_t(r->g_cap);
         c.G.prob = o.guide_prob;
         c.G.min_rough = 0.3f;
         c.G.lo = lo;
@@ -705,6 +719,7 @@ rt_status rt_renderer_render(rt_renderer* r) {
         c.G.rec = training ? r->g_rec.as<float4>() : nullptr;
         if (training) cudaMemsetAsync(r->g_count.ptr, 0, sizeof(int), s);
         c.bounce = 0;
+        if (guided) rtgh::launch_quads(net, gsms, s);
         rth::launch_raygen(c, s);
         if (timed) {  // one kernel after the other, each between two timing events
             for (int bnc = 0; bnc < o.max_depth; bnc++) {
@@ -764,7 +779,7 @@ rt_status rt_renderer_render(rt_renderer* r) {
     } else if (plain_waves > 0) {
         if (!r->graph || r->graph_capacity != r->capacity || r->graph_depth != o.max_depth ||
             r->graph_waves != r->segs.ptr || r->graph_ring != int(nwaves) || r->graph_guided != guided ||
-            r->graph_mix != r->g_mix.ptr) {
+            r->graph_mix != r->g_mix.ptr || (guided && !same_network(r->graph_net, net))) {
             if (r->graph) cudaGraphExecDestroy(r->graph);
             r->graph = nullptr;
             cudaGraph_t g = nullptr;
@@ -780,6 +795,7 @@ rt_status rt_renderer_render(rt_renderer* r) {
             r->graph_ring = int(nwaves);
             r->graph_guided = guided;
             r->graph_mix = r->g_mix.ptr;
+            r->graph_net = net;
         }
         for (int64_t w = 0; w < plain_waves; w++) RT_CUDA(cudaGraphLaunch(r->graph, s), "launch wave graph");
     }
