@@ -752,7 +752,17 @@ __global__ void k_collapse(const WideItem* __restrict__ items, const int* __rest
             const int k = cn.count;
             const uint32_t unary = k == 1 ? 1u : (k == 2 ? 3u : 7u);
             node.meta[s] = uint8_t((unary << 5) | uint32_t(tri_off));
-            for (int i = 0; i < k; i++) order[tb + tri_off + i] = ids[cn.first + i];
+            // ascending: of two triangles at exactly the same distance the first
+            // of a leaf is hit, and the partition's atomics leave their order to chance
+            int t[kMaxLeaf];
+            for (int i = 0; i < k; i++) t[i] = ids[cn.first + i];
+            for (int i = 1; i < k; i++)
+                for (int j = i; j > 0 && t[j] < t[j - 1]; j--) {
+                    const int u = t[j];
+                    t[j] = t[j - 1];
+                    t[j - 1] = u;
+                }
+            for (int i = 0; i < k; i++) order[tb + tri_off + i] = t[i];
             tri_off += k;
         } else {
             node.imask |= uint8_t(1u << s);
