@@ -32,6 +32,16 @@ constexpr int kTravMinBlocks = 8;
 constexpr int kStaleTextured = 1 << 30;  // stale.w flag: the slot's mat_tex holds the last hit's material
 
 
+constexpr int kRecF4 = int(kSlotRecord / 16);  // float4s per slot record
+constexpr int kStagePad = kRecF4 + 1;          // per staged record: the 16-byte accesses of a warp hit distinct banks
+
+// 16 bytes from global to shared memory; waited for by copies_done.
+RT_D void copy16_async(float4* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+                 "l"(src) : "memory");
+}
+RT_D void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 RT_D int warp_fetch(int* counter, int lane) {
     int base = 0;
     if (lane == 0) base = atomicAdd(counter, 32);
@@ -98,8 +108,6 @@ RT_D void raygen_slot(const Ctx& c, const WaveParams& W, int slot, float4* rec) 
 }
 
 constexpr int kRaygenBlock = 256;
-constexpr int kRecF4 = int(kSlotRecord / 16);  // float4s per slot record
-constexpr int kStagePad = kRecF4 + 1;          // per staged record: the 16-byte stores of a warp hit distinct banks
 __global__ void __launch_bounds__(kRaygenBlock) k_raygen(Ctx c) {
     int slot = blockIdx.x * blockDim.x + threadIdx.x;
     WaveCtl* ctl = c.wb.ctl;
@@ -243,7 +251,7 @@ RT_D v3 medium_transmittance(const DevMedium* mp, const MedParams& med, v3 o, v3
 // the register budget of the whole kernel, so the common path runs at a
 // lower occupancy when they are compiled in.
 template <bool Stats, bool Full>
-__global__ void __launch_bounds__(kBlock) k_shade(Ctx c) {
+__global__ void __launch_bounds__(kBlock, Full ? 4 : 5) k_shade(Ctx c) {
     WaveCtl* ctl = c.wb.ctl;
     const int cur = c.bounce & 1, nxt = cur ^ 1;
     const int bounce = c.bounce;
@@ -258,6 +266,18 @@ __global__ void __launch_bounds__(kBlock) k_shade(Ctx c) {
     const int lane = threadIdx.x & 31;
     uint32_t nan_paths = 0;
     int budget_hits = 0;  // media walks that ran out of steps (reported as a watchdog error)
+    // The 32 slot records of a warp's batch, copied in and out line by line:
+    // eight lanes move one 128-byte record with one instruction, four records
+    // at a time, where lanes reading their own records' fields touch 32 lines
+    // an instruction (the L1 pipe was 60% busy, most of it with that).  k_shade
+    // a frame: Cornell 0.442 -> 0.375 ms, 1080p spheres 20.1 -> 18.0 ms, the
+    // guided portal's shade and inference 5.32 -> 5.12 ms, media the same.  The
+    // full build needs its bound of 4 blocks for that: without it the compiler
+    // takes 152 registers (3 blocks, media 19.2 -> 22.5 ms).
+    __shared__ float4 stage[kBlock / 32][32 * kStagePad];
+    float4* const st = stage[threadIdx.x >> 5];
+    float4* const rec = st + lane * kStagePad;
+    char* const records = B.ray_o.base - kRecRayO;
     // Sorted queue: item i lies in the bucket whose prefix range holds it.
     __shared__ int prefix[kShadeBuckets + 1];
     const bool sorted = B.sorted != nullptr;
@@ -285,14 +305,24 @@ __global__ void __launch_bounds__(kBlock) k_shade(Ctx c) {
             } else {
                 slot = q[i];
             }
+        }
+#pragma unroll
+        for (int k = 0; k < kRecF4; k++) {
+            const int r = k * 4 + (lane >> 3), s = __shfl_sync(0xffffffffu, slot, r);
+            if (base + r < total)
+                copy16_async(st + r * kStagePad + (lane & 7), records + size_t(s) * kSlotRecord + (lane & 7) * 16);
+        }
+        const uint2 rs = i < total ? B.rng[slot] : make_uint2(0u, 0u);
+        copies_done();
+        __syncwarp();
+        if (i < total) {
             const Segment& sgm = W.seg[find_segment(W, slot)];
             const JobDesc* jd = c.jobs + sgm.job;
             const SceneView& sc = jd->sc;
             const JobParams& jp = jd->job;
-            float4 o4 = B.ray_o[slot], d4 = B.ray_d[slot], th = B.thr[slot], h4 = B.hit[slot];
-            float4 r4 = B.rad[slot];
-            float4 n0 = B.nee0[slot], n1 = B.nee1[slot];
-            uint2 rs = B.rng[slot];
+            float4 o4 = rec[kRecRayO / 16], d4 = rec[kRecRayD / 16], th = rec[kRecThr / 16], h4 = rec[kRecHit / 16];
+            float4 r4 = rec[kRecRad / 16];
+            float4 n0 = rec[kRecNee0 / 16], n1 = rec[kRecNee1 / 16];
             Rng rng;
             rng.state = uint64_t(rs.x) | (uint64_t(rs.y) << 32);
             if (jp.rng == RT_RNG_LCG) {
@@ -368,15 +398,15 @@ __global__ void __launch_bounds__(kBlock) k_shade(Ctx c) {
                 pos = P;
                 in_m = mi.in_medium;
                 out_m = mi.out_medium;
-                B.stale[slot] = make_float4(s.sn.x, s.sn.y, s.sn.z, __int_as_float(stale_mesh));
+                rec[kRecStale / 16] = make_float4(s.sn.x, s.sn.y, s.sn.z, __int_as_float(stale_mesh));
                 if (bounce == 0) {
                     B.aov_a[slot] = make_float4(s.mat->albedo[0], s.mat->albedo[1], s.mat->albedo[2], Ns.x);
                     B.aov_n[slot] = make_float2(Ns.y, Ns.z);
                 }
             } else {
-                float4 st = B.stale[slot];
-                int mesh = __float_as_int(st.w);
-                s.sn = xyz(st);
+                const float4 last = rec[kRecStale / 16];
+                int mesh = __float_as_int(last.w);
+                s.sn = xyz(last);
                 s.front = true;
                 if (mesh < 0)
                     s.mat = nullptr;
@@ -611,23 +641,31 @@ __global__ void __launch_bounds__(kBlock) k_shade(Ctx c) {
                 R[cap] = f4(L, rec_cos);
                 R[2 * cap] = f4(history, 0.0f);
             }
-            B.rad[slot] = f4(radiance, 0.0f);
-            B.nee0[slot] = f4(nee_e, 0.0f);
-            B.nee1[slot] = f4(nee_l, 0.0f);
+            rec[kRecRad / 16] = f4(radiance, 0.0f);
+            rec[kRecNee0 / 16] = f4(nee_e, 0.0f);
+            rec[kRecNee1 / 16] = f4(nee_l, 0.0f);
             B.rng[slot] = make_uint2(uint32_t(rng.state), uint32_t(rng.state >> 32));
             if (cont) {
-                B.ray_o[slot] = f4(pos, 0.0f);
-                B.ray_d[slot] = f4(L, 0.0f);
-                B.thr[slot] = f4(history, pre_pdf);
+                rec[kRecRayO / 16] = f4(pos, 0.0f);
+                rec[kRecRayD / 16] = f4(L, 0.0f);
+                rec[kRecThr / 16] = f4(history, pre_pdf);
             } else if (defer) {  // k_sample's inputs: origin of the next ray and the front-face flag
-                B.ray_o[slot] = f4(pos, s.front ? 1.0f : 0.0f);
-                B.thr[slot] = f4(history, pre_pdf);
+                rec[kRecRayO / 16] = f4(pos, s.front ? 1.0f : 0.0f);
+                rec[kRecThr / 16] = f4(history, pre_pdf);
             }
         }
         // The next items and the places in the three queues come from one atomic
         // instruction of four lanes: one after the other, each was a round trip
         // to L2 of its own in a kernel that mostly waits for memory.
         const unsigned mc = __ballot_sync(0xffffffffu, cont), md = __ballot_sync(0xffffffffu, defer);
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < kRecF4; k++) {  // a path that ends keeps its ray, hit and throughput (pieces 0..3)
+            const int r = k * 4 + (lane >> 3), s = __shfl_sync(0xffffffffu, slot, r);
+            if (base + r < total && ((lane & 4) || ((mc | md) >> r & 1u)))
+                *reinterpret_cast<float4*>(records + size_t(s) * kSlotRecord + (lane & 7) * 16) =
+                    st[r * kStagePad + (lane & 7)];
+        }
         const unsigned m0 = __ballot_sync(0xffffffffu, sh0), m1 = __ballot_sync(0xffffffffu, sh1);
         int* counter = lane == 0 ? &ctl->fetch_shade
                        : lane == 1 ? &ctl->count[nxt] : lane == 2 ? &ctl->sample_count : &ctl->shadow_count[cur];
