@@ -67,8 +67,12 @@ __global__ void k_begin(const JobDesc* __restrict__ jd) {
 }
 
 // ------------------------------------------------------------------ raygen
-// The camera ray of the path in `slot` (devicePrograms.cu:178-180, 214-227): its slot
-// record goes to `rec`, its random state and queue entry to their arrays.
+// The camera ray of the path in `slot` (devicePrograms.cu:178-180, 214-227): origin
+// and direction go to rec[0] and rec[1], its random state and queue entry to their
+// arrays.  The rest of a slot record is the same for every path before its first
+// hit, and k_shade fills it in at bounce 0 (first_record) instead of reading what
+// raygen would have stored: raygen, resolve and the rest of a 1080p frame of 64 spp
+// 5.82 -> 5.08 ms, k_shade 18.0 -> 17.8 ms.
 RT_D void raygen_slot(const Ctx& c, const WaveParams& W, int slot, float4* rec) {
     const WaveBufs& b = c.wb;
     const Segment sg = W.seg[find_segment(W, slot)];
@@ -92,14 +96,8 @@ RT_D void raygen_slot(const Ctx& c, const WaveParams& W, int slot, float4* rec) 
     float sx = (float(ix) + 0.5f + jx) / float(j.width);
     float sy = (float(iy) + 0.5f + jy) / float(j.height);
     v3 dir = normalize(ld3(cam.dir) + (sx - 0.5f) * ld3(cam.hor) + (sy - 0.5f) * ld3(cam.ver));
-    rec[kRecRayO / 16] = f4(ld3(cam.pos), 0.0f);
-    rec[kRecRayD / 16] = f4(dir, 0.0f);
-    rec[kRecHit / 16] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-    rec[kRecThr / 16] = make_float4(1.f, 1.f, 1.f, 0.f);
-    rec[kRecRad / 16] = make_float4(0.f, 0.f, 0.f, 0.f);
-    rec[kRecNee0 / 16] = make_float4(0.f, 0.f, 0.f, 0.f);
-    rec[kRecNee1 / 16] = make_float4(0.f, 0.f, 0.f, 0.f);
-    rec[kRecStale / 16] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+    rec[0] = f4(ld3(cam.pos), 0.0f);
+    rec[1] = f4(dir, 0.0f);
     b.rng[slot] = make_uint2(uint32_t(rng.state), uint32_t(rng.state >> 32));
     b.queue[0][slot] = slot;
     if (c.G.rec != nullptr)
@@ -107,7 +105,18 @@ RT_D void raygen_slot(const Ctx& c, const WaveParams& W, int slot, float4* rec) 
             c.G.rec[(size_t(r) * 4 + 1) * size_t(b.capacity) + slot] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
+// The fields of a slot record that the camera ray and its closest hit leave
+// open: throughput 1, nothing gathered, no hit before.
+RT_D void first_record(float4* rec) {
+    rec[kRecThr / 16] = make_float4(1.f, 1.f, 1.f, 0.f);
+    rec[kRecRad / 16] = make_float4(0.f, 0.f, 0.f, 0.f);
+    rec[kRecNee0 / 16] = make_float4(0.f, 0.f, 0.f, 0.f);
+    rec[kRecNee1 / 16] = make_float4(0.f, 0.f, 0.f, 0.f);
+    rec[kRecStale / 16] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+}
+
 constexpr int kRaygenBlock = 256;
+static_assert(kRecRayO == 0 && kRecRayD == 16, "a camera ray is the first sector of its record");
 __global__ void __launch_bounds__(kRaygenBlock) k_raygen(Ctx c) {
     int slot = blockIdx.x * blockDim.x + threadIdx.x;
     WaveCtl* ctl = c.wb.ctl;
@@ -124,22 +133,22 @@ __global__ void __launch_bounds__(kRaygenBlock) k_raygen(Ctx c) {
         ctl->fetch_sample = 0;
         for (int b = 0; b < kShadeBuckets; b++) ctl->bucket[b] = 0;
     }
-    // A warp's 32 slot records are 4 KB of contiguous memory: they are built
-    // in shared memory and stored as 16-byte pieces by consecutive lanes, so
-    // that every store instruction writes whole lines.
-    __shared__ float4 stage[kRaygenBlock / 32][32 * kStagePad];
+    // The rays are built in shared memory and stored two lanes to a record, so
+    // that every store instruction writes whole 32-byte sectors.
+    __shared__ float4 stage[kRaygenBlock / 32][32 * 3];  // two and one that spreads the banks
     const int lane = threadIdx.x & 31;
     const int slot0 = slot - lane;
     if (slot0 >= W.wave_count) return;  // the whole warp
     float4* st = stage[threadIdx.x >> 5];
-    if (slot < W.wave_count) raygen_slot(c, W, slot, st + lane * kStagePad);
+    if (slot < W.wave_count) raygen_slot(c, W, slot, st + lane * 3);
     __syncwarp();
-    float4* dst = reinterpret_cast<float4*>(c.wb.ray_o.base - kRecRayO) + size_t(slot0) * kRecF4;
+    char* records = c.wb.ray_o.base - kRecRayO;
 #pragma unroll
-    for (int k = 0; k < kRecF4; k++) {
-        const int idx = k * 32 + lane;  // float4 index in the warp's records
-        const int r = idx / kRecF4;
-        if (slot0 + r < W.wave_count) dst[idx] = st[r * kStagePad + idx % kRecF4];
+    for (int k = 0; k < 2; k++) {
+        const int r = k * 16 + (lane >> 1);
+        if (slot0 + r < W.wave_count)
+            *reinterpret_cast<float4*>(records + size_t(slot0 + r) * kSlotRecord + (lane & 1) * 16) =
+                st[r * 3 + (lane & 1)];
     }
 }
 
@@ -306,13 +315,15 @@ __global__ void __launch_bounds__(kBlock, Full ? 4 : 5) k_shade(Ctx c) {
                 slot = q[i];
             }
         }
+        __syncwarp();  // the last batch's records have left the stage
 #pragma unroll
         for (int k = 0; k < kRecF4; k++) {
             const int r = k * 4 + (lane >> 3), s = __shfl_sync(0xffffffffu, slot, r);
-            if (base + r < total)
+            if (base + r < total && (bounce > 0 || (lane & 7) <= kRecHit / 16))
                 copy16_async(st + r * kStagePad + (lane & 7), records + size_t(s) * kSlotRecord + (lane & 7) * 16);
         }
         const uint2 rs = i < total ? B.rng[slot] : make_uint2(0u, 0u);
+        if (bounce == 0) first_record(rec);
         copies_done();
         __syncwarp();
         if (i < total) {
