@@ -269,6 +269,7 @@ __global__ void __launch_bounds__(kBlock, Full ? 4 : 5) k_shade(Ctx c) {
         ctl->fetch_ext = 0;
     }
     const int total = ctl->count[cur];
+    if (int(blockIdx.x) * kBlock >= total) return;  // nothing for the whole block (no_work)
     const int* __restrict__ q = c.wb.queue[cur];
     const WaveBufs& B = c.wb;
     const WaveParams& W = wave_of(c);
@@ -727,6 +728,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_sample(Ctx c) {
         ctl->shadow_count[nxt] = 0;
         for (int b = 0; b < kShadeBuckets; b++) ctl->bucket[b] = 0;
     }
+    if (no_work(total)) return;
     const WaveBufs& B = c.wb;
     const WaveParams& W = wave_of(c);
     const int lane = threadIdx.x & 31;

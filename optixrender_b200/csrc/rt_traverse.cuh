@@ -366,6 +366,13 @@ constexpr int kListMax = 128;    // room of the list; a lane whose triangles do 
 // Threads per block of the persistent traversal kernels.
 constexpr int kTravBlock = 128;
 
+// Whether `total` queue items leave nothing for the calling warp of a
+// persistent kernel: the warps before it in the grid take one batch of 32
+// each.  It ends at once then; at the last bounces' few paths all 4736 warps
+// of a launch otherwise queue for the fetch counter's address.  A viewer's
+// frame (1080p, 1 spp, 25 bounces) 3.78 -> 3.54 ms.
+RT_D bool no_work(int total) { return int(blockIdx.x) * int(blockDim.x) + int(threadIdx.x & ~31u) >= total; }
+
 // The per-thread traversal stack (local memory; a shared-memory stack
 // measured no faster).
 struct TravStack {
@@ -433,6 +440,7 @@ template <bool AnyHit, bool Stats, class Src>
 RT_D void traverse_queue(Src& src, int* fetch_counter, int total, uint32_t& nodes_visited, uint32_t& tris_tested,
                          uint32_t& rays, uint32_t& overflows) {
     constexpr int kRefillLanes = AnyHit ? kRefillLanesAny : kRefillLanesClosest;
+    if (no_work(total)) return;
     __shared__ TravWarp s_warp[kTravBlock / 32];
     const int lane = threadIdx.x & 31;
     TravWarp& w = s_warp[threadIdx.x >> 5];
@@ -566,6 +574,7 @@ constexpr int kPostponePercentAny = 30;
 template <bool AnyHit, bool Stats, int kPostpone, class Src>
 RT_D void traverse_queue_few(Src& src, int* fetch_counter, int total, uint32_t& nodes_visited, uint32_t& tris_tested,
                              uint32_t& rays, uint32_t& overflows) {
+    if (no_work(total)) return;
     constexpr int kRefillLanes = AnyHit ? kRefillLanesAny : kRefillLanesClosest;
     const int lane = threadIdx.x & 31;
     TravStack st;
