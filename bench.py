@@ -40,7 +40,7 @@ NODE_BYTES, TRI_BYTES, RAY_BYTES = 80, 48, 52  # wide node, triangle record, ray
 # launch of this workload, recorded from an ncu capture (the summary and its
 # command are in profiles/); this run does not measure it.  Keyed by the wave
 # size the capture used: a figure for another wave size is not reported.
-RECORDED_EXTEND_DRAM_BYTES = {67108864: 1354235264}
+RECORDED_EXTEND_DRAM_BYTES = {67108864: 1361733168}
 
 
 def parse():
