@@ -524,6 +524,7 @@ RT_D void traverse_queue(Src& src, int* fetch_counter, int total, uint32_t& node
         }
         __syncwarp();
         const int n = min(w.count, kListMax);
+        __syncwarp();  // every lane has the same n before any lists for the next step (a ballot orders no memory)
         const unsigned walking = __ballot_sync(0xffffffffu, more && tbits == 0);
         const unsigned waiting = __ballot_sync(0xffffffffu, !more && listed);
         if (n > 0 && (n >= kTestAt || walking == 0u || __popc(waiting) >= kDrainLanes)) {
