@@ -383,7 +383,9 @@ RT_API rt_status rt_renderer_guide_samples(rt_renderer* r, float* out, int64_t m
  * any hit, terminate on first hit).  rays: n x 8 floats (ox oy oz tmin dx dy dz
  * tmax).  hits: n x 4 floats (t, u, v, primitive id as float bits; id -1 on a
  * miss).  For any-hit queries hits[i*4+3] holds 1 (occluded) or -1 bits.
- * `device_ptrs` nonzero means both buffers are device memory. */
+ * `device_ptrs` nonzero means both buffers are device memory.  Several threads
+ * may query one renderer at once; their kernels run one after the other on its
+ * stream. */
 RT_API rt_status rt_renderer_trace(rt_renderer* r, int32_t any_hit, const float* rays, int64_t n, float* hits,
                                    int32_t device_ptrs);
 

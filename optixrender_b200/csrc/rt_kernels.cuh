@@ -60,7 +60,6 @@ struct WaveCtl {
     int fetch_shadow;
     int error;     // media walks that exhausted their step budget in this render
     int overflow;  // traversal node groups that found the stack full (the BVH depth check keeps this 0)
-    int fetch_query;  // next ray of a ray query (follows overflow: a query clears the two together)
     unsigned long long stats[8];  // extend rays, shadow rays, ext nodes, ext tris, sh nodes, sh tris,
                                   // NaN samples, paths ended by a NaN throughput
     int bucket[kShadeBuckets];    // extend results per shade bucket

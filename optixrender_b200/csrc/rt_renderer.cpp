@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <condition_variable>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -264,6 +265,11 @@ struct rt_renderer {
     std::mutex query_mu;
     DevBuf query_dev;
     void* query_host = nullptr;
+    // Counters of the other ray queries (QueryCounters), behind the control
+    // block: one bit per pair in use by a call.
+    std::mutex counters_mu;
+    std::condition_variable counters_returned;
+    uint64_t counters_used = 0;
     DevBuf q_job, q_wave, q_index, q_ctl;  // rt_renderer_trace_wavefront: its job, wave table and counters
     // one captured wave (raygen, (extend, shade, shadow) x depth, resolve, advance)
     cudaGraphExec_t graph = nullptr;
@@ -445,6 +451,44 @@ int* overflow_counter(rt_renderer* r) {
     return reinterpret_cast<int*>(static_cast<char*>(r->ctl.ptr) + offsetof(WaveCtl, overflow));
 }
 
+// The overflow count and the fetch counter of one ray query, for the time of
+// the call: calls from several threads may queue their clears and kernels on
+// the renderer's stream in any order, and a kernel that finds another call's
+// count in its fetch counter leaves rays out.  A call beyond kQueryCounters
+// waits for one of the others to return.  A pair that comes back is cleared on
+// the same stream, so after everything that its last call queued.
+constexpr int kQueryCounters = 64;
+constexpr size_t kQueryCounterBytes = 16;
+class QueryCounters {
+  public:
+    explicit QueryCounters(rt_renderer* r) : r_(r) {
+        std::unique_lock<std::mutex> lk(r->counters_mu);
+        r->counters_returned.wait(lk, [r] { return r->counters_used != ~uint64_t(0); });
+        index_ = __builtin_ctzll(~r->counters_used);
+        r->counters_used |= uint64_t(1) << index_;
+    }
+    ~QueryCounters() {
+        {
+            std::lock_guard<std::mutex> lk(r_->counters_mu);
+            r_->counters_used &= ~(uint64_t(1) << index_);
+        }
+        r_->counters_returned.notify_one();
+    }
+    QueryCounters(const QueryCounters&) = delete;
+    QueryCounters& operator=(const QueryCounters&) = delete;
+    int* overflow() const {
+        return reinterpret_cast<int*>(static_cast<char*>(r_->ctl.ptr) + sizeof(WaveCtl) +
+                                      size_t(index_) * kQueryCounterBytes);
+    }
+    int* fetch() const { return overflow() + 1; }
+
+  private:
+    rt_renderer* r_;
+    int index_;
+};
+static_assert(kQueryCounters == 64, "one bit per pair in counters_used");
+static_assert(sizeof(WaveCtl) % sizeof(int) == 0, "the counters behind the control block are aligned");
+
 rt_status overflow_status(int n, const char* what) {
     if (n <= 0) return RT_OK;
     return fail(RT_ERR_DEVICE_WATCHDOG, std::string(what) + ": " + std::to_string(n) +
@@ -500,10 +544,11 @@ rt_status rt_renderer_create(const rt_scene* s, const rt_options* opts, rt_rende
     if (st == RT_OK) {
         e = cudaEventCreate(&r->ev0);
         if (e == cudaSuccess) e = cudaEventCreate(&r->ev1);
-        if (e == cudaSuccess) e = cudaMalloc(&r->ctl.ptr, sizeof(WaveCtl));
+        const size_t ctl_bytes = sizeof(WaveCtl) + kQueryCounters * kQueryCounterBytes;
+        if (e == cudaSuccess) e = cudaMalloc(&r->ctl.ptr, ctl_bytes);
         if (e == cudaSuccess) {
-            r->ctl.bytes = sizeof(WaveCtl);
-            e = cudaMemset(r->ctl.ptr, 0, sizeof(WaveCtl));
+            r->ctl.bytes = ctl_bytes;
+            e = cudaMemset(r->ctl.ptr, 0, ctl_bytes);
         }
         if (e == cudaSuccess) e = r->job.alloc(sizeof(JobDesc));
         if (e != cudaSuccess) st = cuda_fail(e, "rt_renderer_create");
@@ -1036,9 +1081,8 @@ rt_status rt_renderer_trace(rt_renderer* r, int32_t any_hit, const float* rays, 
         rt_status st;
         if (trace_small(r, any_hit != 0, rays, n, hits, st)) return st;
     }
-    int* ovf = overflow_counter(r);
-    int* fetch = ovf + 1;
-    static_assert(offsetof(WaveCtl, fetch_query) == offsetof(WaveCtl, overflow) + sizeof(int), "counter layout");
+    const QueryCounters counters(r);
+    int *ovf = counters.overflow(), *fetch = counters.fetch();
     int h_ovf = 0;
     RT_CUDA(cudaMemsetAsync(ovf, 0, 2 * sizeof(int), r->stream), "rt_renderer_trace");
     if (device_ptrs) {
