@@ -137,7 +137,14 @@ RT_D uint32_t hle2_mask(uint32_t a, uint32_t b) {  // 0xFFFF in the lanes with a
 // are scaled down to that length.  That keeps every box the ray meets: signs
 // stay, near planes only come nearer, and a far plane ahead by 0.25 steps or
 // more, which is added to E there, stays beyond the shortest slab's end, where
-// the ray has left the node.  Distances beyond 1e30 report every slot.
+// the ray has left the node.  (c / |s| comes first there: lim / |s| can fall
+// below the smallest float.)  Distances beyond 1e30 report every slot.
+// Long directions (queries ask for no unit length) make short distances: k is
+// bounded (mx >= 2^-102), so that 2^24 k stays a float and a step below 2^-126,
+// which single precision flushes to zero, puts a plane off by at most
+// 255 * 2^-126 k = 2^-26, within E.  Slabs of less than 2^-114 lose precision
+// for it, and below 2^-115 every slot is reported: at 2^-118 the flushed steps
+// leave nothing to tell the planes apart by.
 RT_D uint32_t intersect_children(const CwNode* nodes, uint32_t idx, const TravRay& r, float tmax, uint32_t& child_base,
                                  uint32_t& tri_base, uint32_t& imask, uint32_t& meta_lo, uint32_t& meta_hi) {
     const float4* q = reinterpret_cast<const float4*>(nodes + idx);
@@ -158,16 +165,17 @@ RT_D uint32_t intersect_children(const CwNode* nodes, uint32_t idx, const TravRa
     cx -= t0, cy -= t0, cz -= t0;
     float mx = max3f(fabsf(sx), fabsf(sy), fabsf(sz));
     const float lim =
-        1024.0f * max3f(min3f(fabsf(sx), fabsf(sy), fabsf(sz)), fabsf(t0) * 0x1p-28f, 0x1p-90f);
+        1024.0f * max3f(min3f(fabsf(sx), fabsf(sy), fabsf(sz)), fabsf(t0) * 0x1p-28f, 0x1p-112f);
     float wide = 0.4f * 0x1p-24f;
     const bool far_out = !(fmaxf(mx, fabsf(t0)) < 1e30f);
     if (mx > lim) {
         wide = 0.65f * 0x1p-24f;
         mx = lim;
-        if (fabsf(sx) > lim) cx *= lim / fabsf(sx), sx = copysignf(lim, sx);
-        if (fabsf(sy) > lim) cy *= lim / fabsf(sy), sy = copysignf(lim, sy);
-        if (fabsf(sz) > lim) cz *= lim / fabsf(sz), sz = copysignf(lim, sz);
+        if (fabsf(sx) > lim) cx = cx / fabsf(sx) * lim, sx = copysignf(lim, sx);
+        if (fabsf(sy) > lim) cy = cy / fabsf(sy) * lim, sy = copysignf(lim, sy);
+        if (fabsf(sz) > lim) cz = cz / fabsf(sz) * lim, sz = copysignf(lim, sz);
     }
+    mx = fmaxf(mx, 0x1p-102f);
     const uint32_t kb = (244u << 23) - (__float_as_uint(mx) & 0x7F800000u);  // k mx in [2^-10, 2^-9)
     const float k = __uint_as_float(kb), k24 = __uint_as_float(kb + (24u << 23));
     sx *= k24, sy *= k24, sz *= k24;
