@@ -123,7 +123,7 @@ struct Ctx {
     int max_depth;  // largest max_depth of the jobs in the wave
     rtg::GuideCtx G;  // path guiding (G.mix null: not guided)
     int features;     // kFeature* bits of the wave's scenes and jobs (host side: picks the shade kernel)
-    int few_nodes;    // few_nodes() of all the wave's scenes (host side: picks the traversal loop)
+    int few_nodes;    // few_nodes() of the wave's scene, or few_loop() of its scenes (host side: picks the traversal loop)
 };
 
 // Scenes whose rays visit a node or two and test triangles at each of them are

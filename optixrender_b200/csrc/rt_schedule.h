@@ -36,6 +36,15 @@ struct PlanState {
     size_t group_rr = 0; // rotation point over the groups (fair)
 };
 
+// Whether a wave runs the traversal loop for scenes of few nodes (few_nodes in
+// rt_kernels.cuh): with so many paths in such scenes and in larger ones.  Both
+// loops answer every scene.  2^23 paths cost, few / large loop: Cornell 7.00 /
+// 7.31 ms, the 2.59M-triangle spheres 10.34 / 9.38 ms, so a path of a large
+// scene gains three times what one of a small scene loses; 7 : 1 of the two
+// 8.69 / 8.60, 6 : 2 8.98 / 8.73, 4 : 4 9.46 / 8.98 ms; textured 7.98 / 8.30,
+// media 14.39 / 14.36, 6 : 2 10.77 / 10.88, 4 : 4 12.05 / 12.10 ms.
+inline bool few_loop(int64_t few_paths, int64_t large_paths) { return few_paths >= 3 * large_paths; }
+
 // Returns (index into `jobs`, paths) per segment; all segments share one group.
 inline std::vector<std::pair<size_t, int64_t>> plan_wave(const std::vector<PlanJob>& jobs, int policy,
                                                          int64_t capacity, int max_segments, PlanState& st) {

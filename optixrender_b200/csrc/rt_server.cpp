@@ -37,6 +37,7 @@
 #include <memory>
 #include <mutex>
 #include <thread>
+#include <tuple>
 #include <vector>
 
 #include "rt_guide_host.h"
@@ -106,7 +107,6 @@ struct rt_server {
     std::vector<std::unique_ptr<DeviceScene>> scenes;
     std::vector<SceneGuide> guides;  // one per scene; networks created at the first guided wave
     int64_t scene_bytes = 0;
-    bool few = true;                  // few_nodes() of every resident scene
     std::vector<int> scene_features;  // per scene: kFeatureMedia / kFeatureTextures
     std::map<int64_t, std::unique_ptr<Job>> jobs;
     std::deque<int64_t> queued;
@@ -129,7 +129,8 @@ struct rt_server {
     std::vector<cudaEvent_t> ring_ev;     // end of the wave in each ring slot
     std::vector<cudaEvent_t> ring_start;  // its start, for the device-busy time
     std::vector<char> ring_timed;         // slot holds a wave not yet added to busy_ms
-    std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // by (bounce count, guided scene + 1 or 0)
+    // by bounce count, group and traversal loop (few_loop)
+    std::map<std::tuple<int, int, bool>, cudaGraphExec_t> graphs;
     rth::LaunchShape shape{};
     // stats
     int64_t waves = 0, paths = 0, done = 0, submitted = 0, depth_sum = 0, guided_waves = 0, training_waves = 0;
@@ -252,8 +253,8 @@ int job_group(const rt_server* s, const rt_job_desc& d) {
 }
 
 // `group`: the wave's group; a guided group's wave samples the guiding
-// network of its scene.
-Ctx make_ctx(rt_server* s, int group) {
+// network of its scene.  `few`: its traversal loop (few_loop).
+Ctx make_ctx(rt_server* s, int group, bool few) {
     const int gscene = group >= kGroupGuided0 ? group - kGroupGuided0 : -1;
     Ctx c;
     std::memset(&c, 0, sizeof(c));
@@ -284,7 +285,7 @@ Ctx make_ctx(rt_server* s, int group) {
     c.wave_ring = s->ring_size;
     c.max_depth = s->opt.max_depth;
     c.features = group == kGroupPlain ? 0 : group == kGroupFull ? kFeatureMedia | kFeatureTextures : kFeatureGuide;
-    c.few_nodes = s->few;
+    c.few_nodes = few;
     if (gscene >= 0) {
         const SceneGuide& g = s->guides[size_t(gscene)];
         c.G.mix = s->g_mix.as<float4>();
@@ -333,12 +334,12 @@ void issue_wave(rt_server* s, const Ctx& c0, int depth, int gscene, bool trainin
     rth::launch_next_wave(c, s->stream);
 }
 
-// One captured wave per bounce count: raygen, (extend, shade, shadow) x depth,
+// One captured wave per bounce count, group and traversal loop: raygen, (extend, shade, shadow) x depth,
 // resolve, advance of the wave ring.  A wave uses the graph of the deepest
 // job in it; each path still stops at its own job's max_depth.
-rt_status wave_graph(rt_server* s, int depth, int group, cudaGraphExec_t* out) {
+rt_status wave_graph(rt_server* s, int depth, int group, bool few, cudaGraphExec_t* out) {
     const int gscene = group >= kGroupGuided0 ? group - kGroupGuided0 : -1;
-    const std::pair<int, int> key(depth, group);
+    const std::tuple<int, int, bool> key(depth, group, few);
     auto it = s->graphs.find(key);
     if (it != s->graphs.end()) {
         *out = it->second;
@@ -346,7 +347,7 @@ rt_status wave_graph(rt_server* s, int depth, int group, cudaGraphExec_t* out) {
     }
     cudaGraph_t g = nullptr;
     SV_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin graph capture");
-    issue_wave(s, make_ctx(s, group), depth, gscene, false);
+    issue_wave(s, make_ctx(s, group, few), depth, gscene, false);
     SV_CUDA(cudaStreamEndCapture(s->stream, &g), "end graph capture");
     cudaGraphExec_t ge = nullptr;
     cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
@@ -483,6 +484,7 @@ rt_status step_locked(rt_server* s, int32_t* did_work, cudaEvent_t* blocked) {
     WaveParams wp;
     std::memset(&wp, 0, sizeof(wp));
     int filled = 0, depth = 1;
+    int64_t few_paths = 0;  // of scenes of few nodes
     const int group = plan.empty() ? kGroupPlain : job_group(s, plan.front().first->desc);
     const int gscene = group >= kGroupGuided0 ? group - kGroupGuided0 : -1;
     std::vector<Job*> completing;
@@ -495,11 +497,13 @@ rt_status step_locked(rt_server* s, int32_t* did_work, cudaEvent_t* blocked) {
         g.path_begin = j.issued;
         j.issued += pj.second;
         filled += int(pj.second);
+        if (few_nodes(s->scenes[size_t(j.desc.scene)]->view)) few_paths += pj.second;
         depth = std::max(depth, j.desc.max_depth);
         if (j.issued >= j.total) completing.push_back(&j);
     }
     if (filled > 0) {
         wp.wave_count = filled;
+        const bool few = few_loop(few_paths, filled - few_paths);
         bool training = false;
         if (gscene >= 0) {
             rt_status gs = ensure_guide_buffers(s);
@@ -509,7 +513,7 @@ rt_status step_locked(rt_server* s, int32_t* did_work, cudaEvent_t* blocked) {
         }
         cudaGraphExec_t graph = nullptr;
         if (!training) {
-            rt_status gs = wave_graph(s, depth, group, &graph);
+            rt_status gs = wave_graph(s, depth, group, few, &graph);
             if (gs) return gs;
         }
         int pos = s->ring_pos;
@@ -522,7 +526,7 @@ rt_status step_locked(rt_server* s, int32_t* did_work, cudaEvent_t* blocked) {
             // launched directly: the wave records training samples, then the
             // scene's network takes guide_steps Adam steps on batches of them
             SceneGuide& g = s->guides[size_t(gscene)];
-            issue_wave(s, make_ctx(s, group), depth, gscene, true);
+            issue_wave(s, make_ctx(s, group, few), depth, gscene, true);
             for (int k = 0; k < s->opt.guide_steps; k++) {
                 SV_CUDA(cudaMemsetAsync(s->g_wsum.ptr, 0, sizeof(float), s->stream), "guide batch");
                 rtgh::launch_batch(s->g_buf.as<float4>(), s->g_count.as<int>(), int(s->g_buf.bytes / 32),
@@ -716,12 +720,6 @@ rt_status rt_server_add_scene(rt_server* s, const rt_scene* scene, int32_t* id) 
         SV_CUDA(s->mat_tex.alloc(size_t(s->capacity) * sizeof(DevMaterial)), "allocate textured materials");
         for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);  // captured without the buffer
         s->graphs.clear();
-    }
-    if (s->few && !few_nodes(ds->view)) {
-        SV_CUDA(cudaStreamSynchronize(s->stream), "rt_server_add_scene");
-        for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second);  // captured with the other traversal loop
-        s->graphs.clear();
-        s->few = false;
     }
     s->scene_features.push_back((ds->view.num_media > 0 ? kFeatureMedia : 0) |
                                 (ds->view.num_tex > 0 ? kFeatureTextures : 0));
