@@ -853,8 +853,11 @@ rt_status rt_renderer_render(rt_renderer* r) {
         }
         for (int64_t w = 0; w < plain_waves; w++) RT_CUDA(cudaGraphLaunch(r->graph, s), "launch wave graph");
     }
-    launches += int(nwaves) * (4 * o.max_depth + 3) + (guided ? int(nwaves) * o.max_depth : 0) +
-                int(train_waves) * (1 + 3 * o.guide_steps);
+    // guided: an inference per bounce and the quads; training: the samples, and per
+    // step the batch, its backward and weight-gradient passes and two Adam kernels
+    launches += int(nwaves) * (4 * o.max_depth + 3) +
+                (guided ? int(nwaves) * (o.max_depth + (net.quads ? 1 : 0)) : 0) +
+                int(train_waves) * (1 + 5 * o.guide_steps);
     ext = int(nwaves) * o.max_depth;
     rth::launch_finalize(hj, dj, s);
     launches++;
