@@ -390,11 +390,16 @@ RT_API rt_status rt_renderer_trace(rt_renderer* r, int32_t any_hit, const float*
                                    int32_t device_ptrs);
 
 /* The queries of rt_renderer_trace (host buffers), answered by the path
- * tracer's own persistent traversal kernels instead of a one-thread-per-ray
- * kernel: the batch becomes the extend queue (closest hit) or the shadow
- * queue (any hit) of a one-bounce wave, and the kernels Render() launches for
- * devicePrograms.cu:258-269 and :303-319 run on it with the same launch
- * shape, lane refill and triangle postponing.  Every ray must have tmin =
+ * tracer's own kernels.  rt_renderer_trace takes one thread per ray for
+ * batches that the chip's resident threads hold at once and a persistent loop
+ * with lane refill for larger ones.  Here a batch of any size becomes the
+ * extend queue (closest hit) or the shadow queue (any hit) of a one-bounce
+ * wave, and the kernels Render() launches for devicePrograms.cu:258-269 and
+ * :303-319 run on it with the same launch shape: in scenes of more than 512
+ * wide nodes triangles are tested by the whole warp in the order the ray met
+ * them, as in rt_renderer_trace; in smaller ones a lane may postpone its
+ * triangles, and of two at exactly the same distance another one may be
+ * reported.  Every ray must have tmin =
  * 1e-4 (EPS, core/cuda/Utils.h:10, the offset of every ray the integrator
  * traces) and closest-hit rays tmax = FLT_MAX or +inf (the extend kernel's
  * extent); any-hit rays keep their own tmax.  Other extents give
@@ -409,8 +414,9 @@ RT_API rt_status rt_renderer_trace_wavefront(rt_renderer* r, int32_t any_hit, co
 
 /* rt_renderer_trace with host buffers, for callers that must not allocate
  * device memory during the call (no counterpart in the reference).
- * cudaMalloc and cudaFree, which rt_renderer_trace uses for its per-call
- * buffers, can synchronise the whole device, stalling a render or serving
+ * cudaMalloc and cudaFree, which rt_renderer_trace uses for the buffers of
+ * host queries above 16,384 rays (and for the blocks it keeps for smaller
+ * ones, at the first of them), can synchronise the whole device, stalling a render or serving
  * loop's other streams, and they fail once the caller has taken the remaining
  * device memory for its own pool.  This call allocates nothing: the rays and
  * hits pass through one fixed device array per device (65,536 rays, 3 MiB),

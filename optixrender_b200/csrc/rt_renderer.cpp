@@ -1111,7 +1111,8 @@ rt_status rt_renderer_trace(rt_renderer* r, int32_t any_hit, const float* rays, 
 // the batch is staged as the extend queue (closest hit) or the shadow queue
 // (any hit) of a one-bounce wave and k_extend / k_shadow run on it with the
 // launch shape of Render(), so these hits come from exactly the loop that
-// renders images (lane refill, triangle postponing, near-to-far order).
+// renders images of the scene (traverse_queue, or traverse_queue_few with its
+// postponed triangles).
 rt_status rt_renderer_trace_wavefront(rt_renderer* r, int32_t any_hit, const float* rays, int64_t n, float* hits,
                                       int64_t* counters) {
     if (!r || n < 0 || (n > 0 && (!rays || !hits)))
