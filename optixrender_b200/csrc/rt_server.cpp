@@ -120,7 +120,7 @@ struct rt_server {
     DevBuf slots, aov_a, aov_n, rng, q0, q1, sq, sh_o, sh_d, sorted;  // slots: kSlotRecord bytes per slot
     DevBuf mat_tex;  // per-slot textured materials, once a scene with textures is resident
     // guiding: per-slot mixtures, training records and samples, one batch
-    DevBuf g_mix, g_quads, g_rec, g_buf, g_count, g_wsum, g_bpos, g_bdir, g_bw;
+    DevBuf g_mix, g_rec, g_buf, g_count, g_wsum, g_bpos, g_bdir, g_bw;
     int64_t guide_bytes = 0;
     int capacity = 0;
     int ring_size = 0;
@@ -220,14 +220,7 @@ rt_status ensure_guide_buffers(rt_server* s) {
     SV_CUDA(s->g_bpos.alloc(size_t(kGuideBatch) * 12), "allocate guide batch");
     SV_CUDA(s->g_bdir.alloc(size_t(kGuideBatch) * 12), "allocate guide batch");
     SV_CUDA(s->g_bw.alloc(size_t(kGuideBatch) * 4), "allocate guide batch");
-    {  // the quads of the network a wave samples; every scene's network has the default resolution
-        rtg::NetView net{};
-        rt_guide_options go;
-        rt_guide_options_default(&go);
-        rtgh::level_resolutions(go.max_resolution, net.res);
-        if (s->g_quads.alloc(rtgh::quad_layout(net)) != cudaSuccess) cudaGetLastError();  // no room: read the table
-    }
-    s->guide_bytes = int64_t(s->g_mix.bytes + s->g_quads.bytes + s->g_rec.bytes + s->g_buf.bytes + 3 * size_t(kGuideBatch) * 12);
+    s->guide_bytes = int64_t(s->g_mix.bytes + s->g_rec.bytes + s->g_buf.bytes + 3 * size_t(kGuideBatch) * 12);
     return RT_OK;
 }
 
@@ -310,7 +303,12 @@ void issue_wave(rt_server* s, const Ctx& c0, int depth, int gscene, bool trainin
         const SceneGuide& g = s->guides[size_t(gscene)];
         net = guide_view(g.net, g.lo, g.inv);
         gsms = guide_sms(g.net);
-        if (rtgh::quad_layout(net) <= s->g_quads.bytes) net.quads = s->g_quads.as<uint4>();
+        // The quads lie in the sample buffer, which holds nothing between the
+        // last batch of a training wave and the samples at the next one's end:
+        // memory of their own would count against the budget (18 MB at the
+        // default resolution).  A server of waves below 2^17.5 paths has no
+        // room there and its inference reads the table.
+        if (rtgh::quad_layout(net) <= s->g_buf.bytes) net.quads = s->g_buf.as<uint4>();
         rtgh::launch_quads(net, gsms, s->stream);
     }
     if (training) cudaMemsetAsync(s->g_count.ptr, 0, sizeof(int), s->stream);
